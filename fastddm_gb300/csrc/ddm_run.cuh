@@ -20,9 +20,13 @@ inline void split_ff(double d, float& h, float& l) {
 
 constexpr size_t kMaxDynSmem = 232448;  // 227 KB opt-in limit per CTA on sm_100-class parts
 
-template <class K> inline cudaError_t allow_smem(K kernel, size_t bytes) {
-  if (bytes <= 48 * 1024) return cudaSuccess;
-  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+// Opts a kernel in to `bytes` of dynamic shared memory where they and its static part (the many-job
+// kernels': kListStaticSmem) pass the 48 KB of a plain launch.  The limit is always set to the most the kernel
+// can have, so a call in one thread never lowers it between another's call of this and its launch.
+template <class K> inline cudaError_t allow_smem(K kernel, size_t bytes, size_t static_bytes = 0) {
+  if (bytes + static_bytes <= 48 * 1024) return cudaSuccess;
+  if (bytes + static_bytes > kMaxDynSmem) return cudaErrorInvalidValue;
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kMaxDynSmem - static_bytes));
 }
 
 // Threads per CTA of the temporal kernels: about one radix-8 butterfly per
@@ -714,7 +718,7 @@ template <class S, class A>
 int run_temporal_list_t(const TemporalListGroup& g, cudaStream_t st, std::string& err) {
   if (g.nitems <= 0) return 0;
   auto go = [&](auto kernel) -> int {
-    cudaError_t ce = allow_smem(kernel, g.smem);
+    cudaError_t ce = allow_smem(kernel, g.smem, kListStaticSmem);
     int occ = 0, dev = 0, nsm = 0;
     if (ce == cudaSuccess) ce = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, g.threads, g.smem);
     if (ce == cudaSuccess) ce = cudaGetDevice(&dev);
