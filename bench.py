@@ -488,6 +488,14 @@ class ClockSampler:
 
 
 # ---------------------------------------------------------------------------
+def side_record(f, *args):
+    """A record beside the headline: an error in it is recorded, and the line still comes out."""
+    try:
+        return f(*args)
+    except (ValueError, RuntimeError) as e:
+        return {"error": f"{type(e).__name__}: {e}"}
+
+
 def dist_setup():
     from fastddm_gb300 import replicas
 
@@ -704,11 +712,10 @@ def run_ours(args):
     # the azimuthal average of the timed result (512 bins), both kernel orders
     azavg = fits = None
     if rank == 0 and not args.no_check:
-        azavg, aa_obj = azavg_record(out, nx, ny, device)
-        try:
-            fits = fit_record(aa_obj, np.asarray(lags, dtype=np.float64))
-        except (ValueError, RuntimeError) as e:  # recorded, not fatal to the structure-function line
-            fits = {"error": f"{type(e).__name__}: {e}"}
+        rec = side_record(azavg_record, out, nx, ny, device)
+        azavg, aa_obj = rec if isinstance(rec, tuple) else (rec, None)
+        if aa_obj is not None:
+            fits = side_record(fit_record, aa_obj, np.asarray(lags, dtype=np.float64))
 
     # end to end through the public API: pinned host frames in, host result out
     e2e = None
@@ -790,7 +797,7 @@ def run_ours(args):
     if rank == 0 and ws == 1 and not args.no_serve and args.config == "large":
         del frames
         torch.cuda.empty_cache()
-        serve = serve_records(args, args.requests, device)
+        serve = side_record(serve_records, args, args.requests, device)
 
     if rank == 0:
         line = {
@@ -938,10 +945,7 @@ def run_batch(args):
     seq_ms = min(seq)
     identical = all(bool(torch.equal(a, j.out)) for a, j in zip(batch_out, jobs))
     del plans, batch_out
-    try:
-        fits = batch_fit_record(jobs, device)
-    except (ValueError, RuntimeError) as e:  # recorded, not fatal to the batch line
-        fits = {"error": f"{type(e).__name__}: {e}"}
+    fits = side_record(batch_fit_record, jobs, device)
     line = {
         "metric": "DDM frames/s (batched uneven stacks)", "value": value, "unit": "frames/s", "n_gpus": 1,
         "steps": args.steps, "warmup": args.warmup, "ms_per_step": ms, "higher_is_better": True, "scaling": "weak",
