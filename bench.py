@@ -16,6 +16,7 @@ alone).
 from __future__ import annotations
 
 import argparse
+import importlib.util
 import json
 import math
 import os
@@ -45,9 +46,18 @@ CONFIGS = {
 }
 
 
-def lags_for(name: str, T: int) -> np.ndarray:
-    from fastddm_gb300 import lags as lg
+def module_alone(name: str):
+    """A plain Python module of the package (scenes, lags, FFT lengths, ranks) without the package around it,
+    whose import loads the library: the reference arm runs without any of that."""
+    if f"alone_{name}" not in sys.modules:
+        spec = importlib.util.spec_from_file_location(f"alone_{name}", ROOT / "fastddm_gb300" / f"{name}.py")
+        sys.modules[spec.name] = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(sys.modules[spec.name])
+    return sys.modules[f"alone_{name}"]
 
+
+def lags_for(name: str, T: int) -> np.ndarray:
+    lg = module_alone("lags")
     if name in ("large", "large_tall", "long"):
         return np.unique(lg.logspace_int(T - 1, num=200, endpoint=True))
     return np.arange(1, T)
@@ -513,15 +523,13 @@ def run_reference(args):
     (FFTW 3.3.10) builds only through CMake with a generated config.h, and its
     sources are not present where this benchmark runs.
     """
-    ws, rank, _ = dist_setup()
+    _, rank, _ = module_alone("replicas").world()
     if rank != 0:
         return
     from concurrent.futures import ProcessPoolExecutor
     import multiprocessing as mp
 
-    from fastddm_gb300 import synthetic
-    from fastddm_gb300._fftopt import next_fast_len
-
+    synthetic, next_fast_len = module_alone("synthetic"), module_alone("_fftopt").next_fast_len
     scene = getattr(synthetic, CONFIGS[args.config])
     lags = lags_for(args.config, scene.length)
     T, H, W = scene.length, scene.height, scene.width
