@@ -83,3 +83,23 @@ def test_rule(what, usable):
         dist = np.ma.masked_less(dist, 1.0)
     args = az.bin_arguments(dist, bins, None, None, None, None, True)
     assert az._device_bins_usable(dist, args) is usable
+
+
+@pytest.mark.parametrize("shape,bins,weighted,usable", [
+    ((513, 1024), 2, False, False), ((513, 1024), 3, False, False), ((513, 1024), 5, False, False),
+    ((513, 1024), 20, False, True), ((513, 1024), 512, True, True), ((513, 1024), 5, True, False),
+    ((65, 128), 10, False, False), ((65, 128), 40, False, True), ((129, 129), 2, False, False),
+])
+def test_bins_that_hold_most_pixels_stay_on_the_host(shape, bins, weighted, usable):
+    """A bin's sums are one chain of additions: a map that falls into one or two bins is slower on the device."""
+    from fastddm_gb300 import azimuthalaverage as az
+
+    ky, kx = np.arange(shape[1]) - shape[1] // 2, np.arange(shape[0])
+    dist = np.hypot(*np.meshgrid(kx, ky)) / shape[0]
+    w = np.random.default_rng(0).uniform(0.0, 1.0, dist.shape) if weighted else None
+    args = az.bin_arguments(dist, bins, None, None, w, None, True)
+    assert az._device_bins_usable(dist, args) is usable
+    # a mask that leaves one pixel in fifty shortens the lists
+    mask = np.random.default_rng(1).random(dist.shape) < 0.02
+    args = az.bin_arguments(dist, bins, None, mask, w, None, True)
+    assert az._device_bins_usable(dist, args) is True
