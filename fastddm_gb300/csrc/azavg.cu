@@ -176,21 +176,30 @@ __global__ void __launch_bounds__(256) k_azavg_warp(const double* __restrict__ d
 }
 
 // Set-up on the device: the bin of every pixel, the lists of the bins' pixels in increasing order (a stable
-// counting sort over chunks of kChunk pixels) and the per-bin sums, added in pixel order as the host's.
+// counting sort over chunks of pixels) and the per-bin sums, added in pixel order as the host's.
 // Bound: launches and the chains of additions (a bin's sum waits for one FP64 addition a pixel).
 // 525,312 pixels, 512 bins: 1.4 ms with the uploads, most of it the copies; numpy's search, sort and
 // sums with the uploads 19 ms.
-constexpr int kChunk = 1024;
+constexpr int kMinChunk = 1024;
 constexpr int kMaxBins = 16384;
+
+// Pixels of a chunk: 1024, or as many more as keep the table of chunks x bins within the pixels' own size (4 bytes
+// each) or 16 MB.  With 1024 throughout, 4096 x 2049 pixels and 16,384 bins took 537 MB of scratch.
+int64_t chunk_pixels(uint64_t npix, uint64_t nbins) {
+  const uint64_t most = npix > (1u << 22) ? npix : (1u << 22);
+  uint64_t chunk = kMinChunk;
+  while ((npix + chunk - 1) / chunk * nbins > most) chunk *= 2;
+  return (int64_t)chunk;
+}
 
 // bin (edges[bin - 1] < dist <= edges[bin]) or -1 for a pixel that takes no part, counted per chunk
 __global__ void __launch_bounds__(256) k_bin_keys(const double* __restrict__ dist, const double* __restrict__ w,
-                                                  const uint8_t* __restrict__ mask, int npix,
+                                                  const uint8_t* __restrict__ mask, int npix, int64_t chunk,
                                                   const double* __restrict__ edges, int nbins, double x_min,
                                                   int32_t* __restrict__ key, int32_t* __restrict__ count) {
   int32_t* mine = count + (size_t)blockIdx.x * nbins;
-  for (int j = threadIdx.x; j < kChunk; j += blockDim.x) {
-    const int64_t p = (int64_t)blockIdx.x * kChunk + j;
+  for (int64_t j = threadIdx.x; j < chunk; j += blockDim.x) {
+    const int64_t p = blockIdx.x * chunk + j;
     if (p >= npix) return;
     const double x = dist[p];
     int lo = 0, hi = nbins;  // first edge not below x; NaN is above every edge
@@ -240,14 +249,15 @@ __global__ void __launch_bounds__(32) k_bin_offsets(int32_t* __restrict__ off, i
 
 // one warp a chunk, 32 pixels at a time: equal keys of a step rank by lane
 __global__ void __launch_bounds__(128) k_bin_scatter(const int32_t* __restrict__ key, int npix, int nchunks,
-                                                     int32_t* __restrict__ next, const int32_t* __restrict__ off,
+                                                     int64_t chunk, int32_t* __restrict__ next, const int32_t* __restrict__ off,
                                                      int nbins, int32_t* __restrict__ pix) {
   const int lane = threadIdx.x & 31;
   const int64_t c = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (c >= nchunks) return;  // whole warps leave together
   int32_t* mine = next + (size_t)c * nbins;
-  for (int j = 0; j < kChunk; j += 32) {
-    const int64_t p = c * kChunk + j + lane;
+  const int64_t end = min((c + 1) * chunk, (int64_t)npix);
+  for (int64_t p0 = c * chunk; p0 < end; p0 += 32) {
+    const int64_t p = p0 + lane;
     const int k = p < npix ? key[p] : -1;
     const unsigned same = __match_any_sync(0xffffffffu, k);
     const int rank = __popc(same & ((1u << lane) - 1u));
@@ -344,9 +354,10 @@ extern "C" int fddm_b200_azimuthal_average(const double* d_data, uint64_t nrows,
 extern "C" int fddm_b200_azimuthal_bins_workspace(uint64_t npix, uint64_t nbins, size_t* bytes) {
   fddm::set_last_error("");
   if (!bytes) return fddm::fail_with(FDDM_ERR_INVALID, "null pointer argument");
-  if (npix == 0 || nbins == 0 || npix >= (1ull << 31) - kChunk || nbins > (uint64_t)kMaxBins)
+  if (npix == 0 || nbins == 0 || npix >= (1ull << 31) - kMinChunk || nbins > (uint64_t)kMaxBins)
     return fddm::fail_with(FDDM_ERR_UNSUPPORTED, "azimuthal bins: no pixels or bins, 2^31 pixels or more than 16384 bins");
-  *bytes = (npix + (npix + kChunk - 1) / kChunk * nbins) * sizeof(int32_t);
+  const uint64_t chunk = (uint64_t)chunk_pixels(npix, nbins);
+  *bytes = (npix + (npix + chunk - 1) / chunk * nbins) * sizeof(int32_t);
   return FDDM_OK;
 }
 
@@ -362,15 +373,16 @@ extern "C" int fddm_b200_azimuthal_bins(const double* d_dist, const double* d_we
     return fddm::fail_with(FDDM_ERR_INVALID, "null pointer argument");
   if (workspace_bytes < need) return fddm::fail_with(FDDM_ERR_NOMEM, "azimuthal bins: workspace too small");
   const cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const int n = (int)npix, nb = (int)nbins, nchunks = (n + kChunk - 1) / kChunk;
+  const int64_t chunk = chunk_pixels(npix, nbins);
+  const int n = (int)npix, nb = (int)nbins, nchunks = (int)((npix + chunk - 1) / chunk);
   int32_t* key = static_cast<int32_t*>(d_workspace);
   int32_t* count = key + npix;
   cudaError_t ce = cudaMemsetAsync(count, 0, (size_t)nchunks * nbins * sizeof(int32_t), st);
   if (ce != cudaSuccess) return fddm::fail_with(FDDM_ERR_CUDA, cudaGetErrorString(ce));
-  k_bin_keys<<<nchunks, 256, 0, st>>>(d_dist, d_weight, d_mask, n, d_edges, nb, x_min, key, count);
+  k_bin_keys<<<nchunks, 256, 0, st>>>(d_dist, d_weight, d_mask, n, chunk, d_edges, nb, x_min, key, count);
   k_bin_scan<<<(nb + 31) / 32, 32, 0, st>>>(count, nchunks, nb, d_bin_offsets + 1);
   k_bin_offsets<<<1, 32, 0, st>>>(d_bin_offsets, nb);
-  k_bin_scatter<<<(nchunks + 3) / 4, 128, 0, st>>>(key, n, nchunks, count, d_bin_offsets, nb, d_bin_pixels);
+  k_bin_scatter<<<(nchunks + 3) / 4, 128, 0, st>>>(key, n, nchunks, chunk, count, d_bin_offsets, nb, d_bin_pixels);
   k_bin_sums<<<nb, 32, 0, st>>>(d_dist, d_weight, d_weight2, d_bin_offsets, d_bin_pixels, d_sumw, d_bias, d_mean);
   ce = cudaGetLastError();
   if (ce != cudaSuccess) return fddm::fail_with(FDDM_ERR_CUDA, cudaGetErrorString(ce));

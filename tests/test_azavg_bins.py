@@ -103,3 +103,42 @@ def test_bins_that_hold_most_pixels_stay_on_the_host(shape, bins, weighted, usab
     mask = np.random.default_rng(1).random(dist.shape) < 0.02
     args = az.bin_arguments(dist, bins, None, mask, w, None, True)
     assert az._device_bins_usable(dist, args) is True
+
+
+@pytest.mark.parametrize("npix", [1, 4096, 525312, 4096 * 2049, 30000 * 20000])
+@pytest.mark.parametrize("bins", [1, 513, 16384])
+def test_scratch_is_bounded(npix, bins):
+    """The chunk table stays within the pixels' own size or 16 MB."""
+    import ctypes
+
+    from fastddm_gb300 import _build, _lib
+
+    _build.build()
+    need = ctypes.c_size_t()
+    _lib.check(_lib.load().fddm_b200_azimuthal_bins_workspace(npix, bins, ctypes.byref(need)))
+    assert 4 * npix < need.value <= 4 * npix + max(4 * npix, 1 << 24)
+
+
+@pytest.mark.gpu
+@pytest.mark.skipif(not gpu_ready(), reason="needs a CUDA GPU")
+@pytest.mark.parametrize("form", ["plain", "masked"])
+@pytest.mark.parametrize("n,bins", [(262145, 16384), (300001, 16384), (1100000, 16384), (1100000, 9000)])
+def test_longer_chunks(built_lib, n, bins, form):
+    """Chunks of more than 1024 pixels (2048 and up), ragged last ones among them."""
+    test_device_bins(built_lib, n, bins, form)
+
+
+def test_host_setup_where_device_memory_runs_out(monkeypatch):
+    torch = pytest.importorskip("torch")
+    from fastddm_gb300 import azimuthalaverage as az
+
+    def full(*_):
+        raise torch.OutOfMemoryError("CUDA out of memory")
+
+    monkeypatch.setattr(az, "_bins_on_device", full)
+    dist, edges, rng_, mask, weights, counts = _case(9000, 40, "masked", 0)
+    args = az.bin_arguments(dist, edges, rng_, mask, weights, counts, True)
+    assert az._device_bins_usable(dist, args)
+    tables, setup = az._bin_tables(dist, args, True, torch.device("cpu"))
+    np.testing.assert_array_equal(tables.sum_wi.numpy(), setup.sum_wi)
+    assert int(tables.offsets[-1]) == int(setup.valid.sum())
