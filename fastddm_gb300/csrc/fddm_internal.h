@@ -92,6 +92,7 @@ struct TemporalArgs {
   float fx_beta;
   int fx_headroom;         // whole bits between that and 2^31: the unit of the squares is finer by as much
   float fx_power_sum;
+  float fx_pair_sum;       // long series: from sum |x|^2 over the inputs of a pair of sub-transforms to the sum of its powers
   long long fx_kappa_m;    // mantissa, 2^61 <= m < 2^62
   int fx_kappa_e;          // factor m 2^(e - 62)
 };

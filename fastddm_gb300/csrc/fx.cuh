@@ -111,12 +111,16 @@ __device__ __forceinline__ cx<fx> fx_twmul_inv(cx<fx> v, fxw w, fxc c) {
   return fx_twmul({fx_twice(v.r), fx_twice(v.i)}, w, c);
 }
 
-// v / 2, the first output of a twiddled forward pass
-__device__ __forceinline__ fx fx_half(fx a) {
-  const int h = a.h >> 1;
+// v / 2, the first output of a twiddled forward pass.  A half goes down; or (NEAR) to the side that draws the low
+// word to zero: always down, the low words of a long series' lowest frequencies grow to tens of units from pass
+// to pass, and their roundings with them (20,000 frames of 32 x 32, 48 movies: 2-norm error of D 6.3e-15 down,
+// 5.0e-15 near, 5.2e-15 in float-float).  The shorter series' error is below float-float's either way (4000
+// frames: 3.7e-15 and 3.2e-15 against 5.6e-15), and near took 0.4 to 1 % of their time.
+template <bool NEAR> __device__ __forceinline__ fx fx_half(fx a) {
+  const int h = (NEAR ? iadd(a.h, 1 + ((int)__float_as_uint(a.l) >> 31)) : a.h) >> 1;
   return {h, __fmaf_rn(a.l, 0.5f, __int2float_rn(isub(a.h, iadd(h, h))) * 0.5f)};
 }
-__device__ __forceinline__ cx<fx> fx_half(cx<fx> a) { return {fx_half(a.r), fx_half(a.i)}; }
+template <bool NEAR> __device__ __forceinline__ cx<fx> fx_half(cx<fx> a) { return {fx_half<NEAR>(a.r), fx_half<NEAR>(a.i)}; }
 
 // a sqrt(1/2)
 __device__ __forceinline__ fx fx_sqrt_half(fx a) {
@@ -230,9 +234,9 @@ template <int R> __device__ __forceinline__ void fx_dft_halfzero(cx<fx>* v) {
 
 // ---------------------------------------------------------------------------
 // In-place passes over `nfft` transforms of length n in swizzled shared memory (the
-// counterparts of fft.cuh's; same positions, same digit-reversed order)
+// counterparts of fft.cuh's; same positions, same digit-reversed order).  NEAR as in fx_half.
 // ---------------------------------------------------------------------------
-template <int R, bool INV>
+template <int R, bool INV, bool NEAR>
 __device__ __forceinline__ void fx_pass(cx<fx>* __restrict__ buf, int nfft, int ld, int n, int M, unsigned rs,
                                         unsigned rb, const void* __restrict__ table, int tid, int nthr) {
   const int stride = M / R, bpf = n / R;
@@ -255,7 +259,7 @@ __device__ __forceinline__ void fx_pass(cx<fx>* __restrict__ buf, int nfft, int 
         fx_dft<R, true>(v);
       } else {
         fx_dft<R, false>(v);
-        v[0] = fx_half(v[0]);
+        v[0] = fx_half<NEAR>(v[0]);
 #pragma unroll
         for (int m = 1; m < R; ++m) v[m] = fx_twmul(v[m], w[(m - 1) * stride], c[(m - 1) * stride]);
       }
@@ -303,8 +307,8 @@ __device__ __forceinline__ void fx_pass_two(cx<fx>* __restrict__ buf, int n, con
     for (int r = 0; r < R; ++r) u[r] = buf[n + fx_slots<R, M>::at(sb, r)];
     fx_dft<R, false>(v);
     fx_dft<R, false>(u);
-    buf[sb] = fx_half(v[0]);
-    buf[n + sb] = fx_half(u[0]);
+    buf[sb] = fx_half<false>(v[0]);
+    buf[n + sb] = fx_half<false>(u[0]);
 #pragma unroll
     for (int m = 1; m < R; ++m) {
       const fxw wm = w[(m - 1) * S];
@@ -336,21 +340,21 @@ __device__ __forceinline__ void fx_pass_inverse(cx<fx>* __restrict__ buf, int n,
   }
 }
 
-template <bool INV>
+template <bool INV, bool NEAR = false>
 __device__ __forceinline__ void fx_pass_dispatch(cx<fx>* buf, int nfft, int ld, const FftPlan& p, int s, int tid,
                                                  int nthr) {
   const int n = p.n, M = p.block[s];
   const unsigned rs = p.rstride[s], rb = p.rbpf[s];
   const void* t = p.ptw[s];
   switch (p.radix[s]) {
-    case 2: fx_pass<2, INV>(buf, nfft, ld, n, M, rs, rb, t, tid, nthr); break;
-    case 4: fx_pass<4, INV>(buf, nfft, ld, n, M, rs, rb, t, tid, nthr); break;
-    case 8: fx_pass<8, INV>(buf, nfft, ld, n, M, rs, rb, t, tid, nthr); break;
-    case 3: fx_pass<3, INV>(buf, nfft, ld, n, M, rs, rb, t, tid, nthr); break;
-    case 5: fx_pass<5, INV>(buf, nfft, ld, n, M, rs, rb, t, tid, nthr); break;
-    case 7: fx_pass<7, INV>(buf, nfft, ld, n, M, rs, rb, t, tid, nthr); break;
-    case 11: fx_pass<11, INV>(buf, nfft, ld, n, M, rs, rb, t, tid, nthr); break;
-    case 13: fx_pass<13, INV>(buf, nfft, ld, n, M, rs, rb, t, tid, nthr); break;
+    case 2: fx_pass<2, INV, NEAR>(buf, nfft, ld, n, M, rs, rb, t, tid, nthr); break;
+    case 4: fx_pass<4, INV, NEAR>(buf, nfft, ld, n, M, rs, rb, t, tid, nthr); break;
+    case 8: fx_pass<8, INV, NEAR>(buf, nfft, ld, n, M, rs, rb, t, tid, nthr); break;
+    case 3: fx_pass<3, INV, NEAR>(buf, nfft, ld, n, M, rs, rb, t, tid, nthr); break;
+    case 5: fx_pass<5, INV, NEAR>(buf, nfft, ld, n, M, rs, rb, t, tid, nthr); break;
+    case 7: fx_pass<7, INV, NEAR>(buf, nfft, ld, n, M, rs, rb, t, tid, nthr); break;
+    case 11: fx_pass<11, INV, NEAR>(buf, nfft, ld, n, M, rs, rb, t, tid, nthr); break;
+    case 13: fx_pass<13, INV, NEAR>(buf, nfft, ld, n, M, rs, rb, t, tid, nthr); break;
     default: break;
   }
 }
@@ -375,7 +379,7 @@ __device__ __forceinline__ void fx_first_pass_padded(cx<fx>* __restrict__ buf, c
       if (R == 2) {  // x_t and x_t w_N^t: nothing is summed, so nothing is scaled
         v[1] = fx_twmul(fx_add(v[1], v[1]), tw[j], tc[j]);
       } else {
-        v[0] = fx_half(v[0]);
+        v[0] = fx_half<false>(v[0]);
 #pragma unroll
         for (int m = 1; m < R; ++m) v[m] = fx_twmul(v[m], tw[(m - 1) * stride + j], tc[(m - 1) * stride + j]);
       }
