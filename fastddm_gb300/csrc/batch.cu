@@ -26,8 +26,8 @@
 namespace {
 
 constexpr int kWorkers = 4;
-// Launches of the many-job kernel in one batch: one per (variant, CTA size), 8 x 3 at most.
-constexpr int kMaxGroups = 24;
+// Launches of the many-job kernel in one batch: one per (variant, CTA size), 9 x 3 at most.
+constexpr int kMaxGroups = 32;
 
 struct Workers {
   cudaStream_t s[kWorkers];
@@ -228,7 +228,7 @@ extern "C" int fddm_b200_batch_create(const fddm_b200_job* jobs, uint64_t njobs,
   auto* d_items = reinterpret_cast<fddm::TemporalItem*>(ws + list_off + up256(njobs * sizeof(fddm::TemporalArgs)));
   int* d_counters = reinterpret_cast<int*>(reinterpret_cast<unsigned char*>(d_items) +
                                            up256(nitems_all * sizeof(fddm::TemporalItem)));
-  for (auto& kv : by_key) {  // at most 8 variants x 3 CTA sizes <= kMaxGroups
+  for (auto& kv : by_key) {  // at most 9 variants x 3 CTA sizes <= kMaxGroups
     const size_t first = items.size();
     fddm::TemporalListGroup g;
     g.variant = kv.first.first;

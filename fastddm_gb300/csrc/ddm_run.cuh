@@ -55,7 +55,7 @@ inline bool plan_is_p2(const FftPlan& p) {
 }
 
 // Temporal kernel of a variant: float-float transforms run in block fixed point (variant K:
-// 2 x 2^K points, 0: any plan), the other tiers' variants are 0 generic, 1 radices 2/4/8, 2 the
+// 2 x 2^K points, 0: any plan, 1: no transform), the other tiers' variants are 0 generic, 1 radices 2/4/8, 2 the
 // fused radix-2 path; FP32 ones run two CTAs per SM.  LIST: the many-job kernel.
 // Calls f(kernel) and returns its result.
 template <class S, class A, bool LIST, class F> auto with_tfft_kernel(int variant, F f) {
@@ -489,7 +489,8 @@ int run_ddm_t(const DdmRequest& r, cudaStream_t st, std::string& err) {
     const char* fz = std::getenv("FDDM_B200_TEMPORAL_FUSED");
     const bool fuse = !(fz && fz[0] == '0');
     if (kind == 0) {
-      if (fuse && ta.pt.lgn >= 7 && ta.pt.lgn <= 13) variant = ta.pt.lgn - 1;
+      if (nl == 0 || T - r.lags[0] <= kDirect) variant = 1;
+      else if (fuse && ta.pt.lgn >= 7 && ta.pt.lgn <= 13) variant = ta.pt.lgn - 1;
     } else if (plan_is_p2(ta.pt) && plan_is_p2(ta.pt2)) {
       variant = fuse && fused_radix2_ok<S>(ta.pt) ? 2 : 1;
     }

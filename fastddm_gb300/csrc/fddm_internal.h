@@ -107,7 +107,8 @@ struct TemporalItem {
 // The temporal stage of one job, set up but not launched (DdmRequest::collect):
 // its arguments and launch shape, and whether the many-job kernel can run it
 // (the shared-memory fft kernel; variant 0 generic, 1 radices 2/4/8, 2 the
-// fused radix-2 path; float-float tier: 0 or K for 2 x 2^K points; -1 other kernels).
+// fused radix-2 path; float-float tier: 0, K for 2 x 2^K points, or 1 for direct sums
+// only; -1 other kernels).
 struct TemporalLaunch {
   TemporalArgs args;
   int threads = 0;
