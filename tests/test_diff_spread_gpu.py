@@ -36,3 +36,22 @@ def test_bright_frames(built_lib, T, form, bits):
     for l, g in zip(lags, got):
         exact = (np.abs(f[l:] - f[:T - l]) ** 2).mean(axis=0)
         assert np.linalg.norm(g - exact) <= 2.0 ** -43 * np.linalg.norm(exact), l
+
+
+# the sum of squares about the mean just below, just above and well above the largest FP32 number
+@pytest.mark.parametrize("largest", [3.37e38, 3.5e38, 1e39])
+def test_energy_beyond_fp32(built_lib, largest):
+    """Finite frames whose energy does not fit in FP32 keep their lags, power spectrum and variance."""
+    import fastddm_gb300 as fddm
+
+    rng = np.random.default_rng(0)
+    T = 33
+    base = rng.standard_normal((T, 1, 1)) + np.zeros((T, 4, 4))
+    scale = np.sqrt(largest / (16.0 * ((base[:, 0, 0] - base[:, 0, 0].mean()) ** 2).sum()))
+    imgs = (base * scale).astype(np.float32)
+    got = fddm.ddm(imgs, [1, 20, 30], mode="diff")._data[:, 2, 0]
+    f = imgs.astype(np.float64).sum(axis=(1, 2)) / 4.0
+    exact = [((f[l:] - f[:T - l]) ** 2).mean() for l in (1, 20, 30)] + [(f ** 2).mean(), ((f - f.mean()) ** 2).mean()]
+    for g, e, pairs in zip(got, exact, (32, 13, 3, 0, 0)):
+        if pairs == 0 or e * pairs < 3e38:  # a lag's own sum is a float-float one
+            assert abs(g - e) <= 1e-12 * e
