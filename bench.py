@@ -220,28 +220,39 @@ def time_tier(DdmPlan, mode, T, H, W, code, lags, nx, ny, nt, window, precision,
             "steps": steps}
 
 
-def azavg_record(out, nx: int, ny: int, device, bins: int = 512, reps: int = 3) -> dict:
-    """The azimuthal average of the timed result (``bins`` bins over (0, ky[-1])), both kernel orders.
-
-    Times the host set-up (bin search, weights, per-bin sums) and the device
-    call (set-up tables to the device, one kernel, results left on the device)
-    with CUDA events, best of `reps`; reports the largest relative difference of
-    the fast order against the bit-exact one.
-    """
-    import torch
-
-    from fastddm_gb300 import azimuthalaverage as aa
-
+def half_plane(nx: int, ny: int):
+    """|k| of the half plane, the pixels' counts in the full one, and the largest ky, as azimuthal_average sets
+    them up."""
     kx = 2 * np.pi * np.fft.fftfreq(nx)[: nx // 2 + 1]
     ky = 2 * np.pi * np.fft.fftshift(np.fft.fftfreq(ny))
     counts = np.full((ny, nx // 2 + 1), 2)
     counts[:, 0] = 1
     counts[:, -1] = 1 if nx % 2 == 0 else 2
     gx, gy = np.meshgrid(kx, ky)
-    t0 = time.perf_counter()
-    setup = aa.bin_setup(np.sqrt(gx ** 2 + gy ** 2), bins, (0, ky[-1]), None, None, counts, True)
-    host_ms = 1000 * (time.perf_counter() - t0)
-    rec = {"bins": bins, "pixels": int(ny * (nx // 2 + 1)), "rows": int(out.shape[0]), "host_setup_ms": host_ms}
+    return np.sqrt(gx ** 2 + gy ** 2), counts, ky[-1]
+
+
+def azavg_record(out, nx: int, ny: int, device, bins: int = 512, reps: int = 3) -> dict:
+    """The azimuthal average of the timed result (``bins`` bins over (0, ky[-1])), both kernel orders.
+
+    Times the set-up as a call makes it (edges and weights on the host, bins, lists and
+    per-bin sums on the device) and the average (one kernel, results left on the
+    device), best of `reps`; reports the largest relative difference of the fast
+    order against the bit-exact one.
+    """
+    import torch
+
+    from fastddm_gb300 import azimuthalaverage as aa
+
+    k, counts, k_max = half_plane(nx, ny)
+    rec = {"bins": bins, "pixels": int(ny * (nx // 2 + 1)), "rows": int(out.shape[0]), "setup_ms": float("inf")}
+    for _ in range(reps):
+        torch.cuda.synchronize(device)
+        t0 = time.perf_counter()
+        args = aa.bin_arguments(k, bins, (0, k_max), None, None, counts, True)
+        tables, _ = aa._bin_tables(k, args, True, device)
+        torch.cuda.synchronize(device)
+        rec["setup_ms"] = min(rec["setup_ms"], 1000 * (time.perf_counter() - t0))
     res = {}
     stream = torch.cuda.current_stream(device)
     for label, exact in (("exact", True), ("fast", False)):
@@ -249,7 +260,7 @@ def azavg_record(out, nx: int, ny: int, device, bins: int = 512, reps: int = 3) 
         for _ in range(reps):
             e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
             e0.record(stream)
-            avg, err = aa._run_device(out, setup, True, device, exact, host=False)
+            avg, err = aa._average(out, tables, args.n_bins, True, device, exact, False)
             e1.record(stream)
             torch.cuda.synchronize(device)
             best = min(best, e0.elapsed_time(e1))
@@ -261,8 +272,7 @@ def azavg_record(out, nx: int, ny: int, device, bins: int = 512, reps: int = 3) 
         ok = ~torch.isnan(b)
         diff = max(diff, float(((a[ok] - b[ok]).abs() / b[ok].abs().clamp_min(1e-300)).max()))
     rec["fast_vs_exact_max_rel"] = diff
-    avg, err = res["exact"]
-    return rec, aa.AzimuthalAverage(avg.cpu().numpy(), err.cpu().numpy(), setup.k, None, setup.bin_edges)
+    return rec, device_azavg(out, nx, ny, device, bins)
 
 
 def device_azavg(out, nx: int, ny: int, device, bins: int):
@@ -270,15 +280,9 @@ def device_azavg(out, nx: int, ny: int, device, bins: int):
     (0, ky[-1]), the exact order), as an AzimuthalAverage with tau unset."""
     from fastddm_gb300 import azimuthalaverage as aa
 
-    kx = 2 * np.pi * np.fft.fftfreq(nx)[: nx // 2 + 1]
-    ky = 2 * np.pi * np.fft.fftshift(np.fft.fftfreq(ny))
-    counts = np.full((ny, nx // 2 + 1), 2)
-    counts[:, 0] = 1
-    counts[:, -1] = 1 if nx % 2 == 0 else 2
-    gx, gy = np.meshgrid(kx, ky)
-    setup = aa.bin_setup(np.sqrt(gx ** 2 + gy ** 2), bins, (0, ky[-1]), None, None, counts, True)
-    avg, err = aa._run_device(out, setup, True, device, True, host=True)
-    return aa.AzimuthalAverage(avg, err, setup.k, None, setup.bin_edges)
+    k, counts, k_max = half_plane(nx, ny)
+    avg, err, mean, edges = aa.azimuthal_average_array(out, k, bins, (0, k_max), counts=counts, gpu_id=device.index or 0)
+    return aa.AzimuthalAverage(avg, err, mean, None, edges)
 
 
 def batch_fit_record(jobs, device, sample: int = 4) -> dict:

@@ -313,11 +313,6 @@ def _bin_tables(dist: np.ndarray, args: BinArguments, eval_err: bool, device):
     return _upload_bins(setup, eval_err, device), setup
 
 
-def _run_device(data_dev, setup: BinSetup, eval_err: bool, device, exact: bool = True,
-                host: bool = True):
-    return _average(data_dev, _upload_bins(setup, eval_err, device), setup.n_bins, eval_err, device, exact, host)
-
-
 def _average(data_dev, tables: DeviceBins, n_bins: int, eval_err: bool, device, exact: bool, host: bool):
     nrows = int(data_dev.shape[0])
     npix = int(np.prod(data_dev.shape[1:]))
