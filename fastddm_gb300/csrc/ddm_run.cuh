@@ -456,8 +456,9 @@ int run_ddm_t(const DdmRequest& r, cudaStream_t st, std::string& err) {
           return 4;
         }
         fx_constants(whole, ta);
-        // every pass of a sub-transform but the last halves; the powers' own unit is 2^32
-        ta.fx_pair_sum = (float)std::ldexp((double)ta.M1, -2 * std::max(0, ta.pm.npass - 1) - 32);
+        // every pass of a sub-transform but the last halves; the powers' own unit is 2^32; 2^-10 more for the
+        // rounding of the FP32 sums, which must not come out below the powers'
+        ta.fx_pair_sum = (float)std::ldexp((double)ta.M1 * (1.0 + 1.0 / 1024), -2 * std::max(0, ta.pm.npass - 1) - 32);
         // tables of the first pass and of the half plan's first pass (the one the lags evaluate)
         ta.pt = whole;
         ta.pt.npass = ta.R0 > 2 ? 2 : 1;

@@ -51,3 +51,23 @@ def test_pairs_of_unlike_power(built_lib, monkeypatch, split, kind):
     ref = fddm.ddm(imgs, lags, mode="diff")._data
     rowmax = np.abs(ref).reshape(len(ref), -1).max(axis=1)[:, None, None]
     assert (np.abs(got - ref) <= 1e-8 * np.abs(ref) + 1e-13 * rowmax).all()
+
+
+def test_power_in_one_coefficient(built_lib, monkeypatch):
+    """A whole pair's power in one value, just below and above the powers of two that its shift is chosen by: the
+    inverse passes double it, to just below 2^31."""
+    import fastddm_gb300 as fddm
+
+    monkeypatch.setenv("FDDM_B200_TEMPORAL_SPLIT", "8")
+    T = 512
+    tone = np.exp(2j * np.pi * 32 * np.arange(T) / 1024)
+    # frames whose (0, 1) mode is the tone: two cosines along x, a quarter period apart
+    x = np.exp(2j * np.pi * np.arange(8) / 8)
+    lags = [1, 7, 64, 300, 470]
+    for amplitude in np.linspace(1.0, 2.0, 33):
+        imgs = (amplitude * (tone[:, None, None] * x[None, None, :]).real + np.zeros((T, 4, 8))).astype(np.float32)
+        got = fddm.ddm(imgs, lags, mode="fft")._data[:-2, 2, 1]
+        f = (imgs.astype(np.float64) * np.conj(x)[None, None, :]).sum(axis=(1, 2)) / np.sqrt(32.0)
+        exact = np.array([np.mean(np.abs(f[l:] - f[:T - l]) ** 2) for l in lags])
+        var = np.mean(np.abs(f - f.mean()) ** 2)
+        assert (np.abs(got - exact) <= 16 * 2.0 ** -48 * var * T / (T - np.array(lags)) + 1e-13 * exact).all(), amplitude
