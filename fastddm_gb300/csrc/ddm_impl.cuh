@@ -230,7 +230,7 @@ __global__ void __launch_bounds__(256) k_rows(SpatialArgs a) {
   // different banks
   const int ld = nx + swz_group<S>::G;
   const int lgnx = (nx & (nx - 1)) == 0 ? __ffs(nx) - 1 : -1;
-  const unsigned rnx = div_reciprocal_dev(nx);
+  const unsigned rnx = a.rnx;
   const bool u8_fast = sizeof(IN) == 1 && async_raw && !win && W == nx && lgnx >= 2;
   unsigned char* raw[2] = {smem_raw + (size_t)swz_round<S>(a.pairs_per_block * ld) * sizeof(cx<S>), nullptr};
   raw[1] = raw[0] + a.raw_stage_bytes;
@@ -297,7 +297,7 @@ __global__ void __launch_bounds__(256) k_rows(SpatialArgs a) {
 
     // unpack Z = A + iB into the spectra of the two real rows of each pair,
     // one thread per (k, pair): R[tl][k][2p] and R[tl][k][2p + 1]
-    const unsigned rnp = div_reciprocal_dev(np);
+    const unsigned rnp = np == a.pairs_per_block ? a.rpairs : div_reciprocal_dev(np);
     cx<S>* R = reinterpret_cast<cx<S>*>(a.rbuf) + (size_t)tl * nkx * a.Hpad;
     for (int e = tid; e < np * nkx; e += nthr) {
       const int k = div_by(e, rnp);
@@ -375,7 +375,7 @@ __global__ void __launch_bounds__(512) k_cols(SpatialArgs a) {
   const int nitems = ncg * ((a.tc + TG - 1) / TG);
   const int ld = ny + swz_group<S>::G;  // padded stride: the store phase reads NB transforms at one slot
   cx<S>* bufs[2] = {reinterpret_cast<cx<S>*>(smem_raw), reinterpret_cast<cx<S>*>(smem_raw) + swz_round<S>(NB * ld)};
-  const unsigned rny = div_reciprocal_dev(ny), rTG = div_reciprocal_dev(TG), rCK = div_reciprocal_dev(CK);
+  const unsigned rny = a.rny, rTG = a.rframes, rCK = a.rcols;
   const int tid = threadIdx.x, nthr = blockDim.x;
   const S norm = sc<S>::cst(a.norm_h, a.norm_l, a.norm_d);
   // 1/sqrt(nx ny) is a power of two when nx ny is a power of four: exact scaling

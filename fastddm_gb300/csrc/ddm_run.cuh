@@ -4,6 +4,7 @@
 #include <cmath>
 #include <cstdlib>
 #include <string>
+#include <type_traits>
 #include "ddm_impl.cuh"
 
 namespace fddm {
@@ -111,13 +112,12 @@ cudaError_t launch_rows(const SpatialArgs& a, int items, size_t smem, cudaStream
   return cudaGetLastError();
 }
 
-// Only the FP64 and FP32 tiers instantiate the general kernel's power-of-two variant.  The float-float tier has
-// kernels of its own for power-of-two widths of 32 to 4096 and 8- and 16-bit or float pixels (rows_p2_kernel);
-// its other pixel types and widths of 8, 16 and 8192 take the general variant, whose reciprocal index arithmetic
-// made up for the odd butterflies it carries (64 frames of 1024 x 1024 doubles, the whole call 9.64 -> 8.10 ms).
+// The float-float tier has row kernels of its own for power-of-two widths of 32 to 4096 and 8- and 16-bit or float
+// pixels (rows_p2_kernel), so it instantiates the general kernel's power-of-two variant for the other pixel types
+// only (64 frames of 1024 x 1024 doubles, the whole call 8.09 -> 7.88 ms; 30 frames of 64 x 32 59 -> 58 us).
 template <class S, class IN>
 cudaError_t launch_rows(const SpatialArgs& a, int items, size_t smem, cudaStream_t st) {
-  if constexpr (tier_kind<S>::v != 0)
+  if constexpr (tier_kind<S>::v != 0 || (sizeof(IN) >= 4 && !std::is_same_v<IN, float>))
     if (plan_is_p2(a.px)) return launch_rows<S, IN, true>(a, items, smem, st);
   return launch_rows<S, IN, false>(a, items, smem, st);
 }
@@ -309,6 +309,11 @@ int run_ddm_t(const DdmRequest& r, cudaStream_t st, std::string& err) {
   sa.pairs_per_block = L.pairs_per_block;
   sa.cols_per_block = L.cols_per_block;
   sa.frames_per_block = L.frames_per_block;
+  sa.rnx = div_reciprocal(nx);
+  sa.rny = div_reciprocal(ny);
+  sa.rpairs = div_reciprocal(L.pairs_per_block);
+  sa.rcols = div_reciprocal(L.cols_per_block);
+  sa.rframes = div_reciprocal(L.frames_per_block);
   sa.px = tx.plan; sa.py = ty.plan;
   // float-float tier: kernels of power-of-two sizes, whose plans order the radices differently
   SpatialKernel rows_k = nullptr, cols_k = nullptr;

@@ -37,6 +37,7 @@ struct SpatialArgs {
   int Tpad;              // spectrum row stride (elements)
   int pairs_per_block, cols_per_block, frames_per_block;
   int raw_stage_bytes;   // >0: rows are staged with cp.async (16-byte aligned rows)
+  unsigned rnx, rny, rpairs, rcols, rframes;  // reciprocals (div_reciprocal) of nx, ny and the blocking
   FftPlan px, py;
   const void* twx;
   const void* twy;

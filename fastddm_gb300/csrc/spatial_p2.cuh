@@ -254,7 +254,7 @@ __global__ void __launch_bounds__(256) k_rows_p2(const __grid_constant__ Spatial
     p2_passes_from<LG, 1>(buf, np, a.px, w, tid, nthr);
 
     // twice the spectra of the two real rows of each pair (the column pass's scale halves them)
-    const unsigned rnp = div_reciprocal_dev(np);
+    const unsigned rnp = np == a.pairs_per_block ? a.rpairs : div_reciprocal_dev(np);
     cx<ff>* R = reinterpret_cast<cx<ff>*>(a.rbuf) + (size_t)tl * nkx * a.Hpad;
     for (int e = tid; e < np * nkx; e += nthr) {
       const int k = div_by(e, rnp);
@@ -302,7 +302,7 @@ __global__ void __launch_bounds__(512) k_cols_p2(const __grid_constant__ Spatial
   const int ncg = (nkx + CK - 1) / CK;
   const int nitems = ncg * ((a.tc + TG - 1) / TG);
   cx<ff>* bufs[2] = {reinterpret_cast<cx<ff>*>(smem_raw), reinterpret_cast<cx<ff>*>(smem_raw) + NB * n};
-  const unsigned rTG = div_reciprocal_dev(TG), rCK = div_reciprocal_dev(CK);
+  const unsigned rTG = a.rframes, rCK = a.rcols;
   const int tid = threadIdx.x, nthr = blockDim.x;
   const ff norm = {a.norm_h, a.norm_l};
   // a power-of-two scale (nx ny a power of four) is exact
